@@ -53,13 +53,39 @@ namespace mlp {
 __device__ __forceinline__ double fmadd(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fmadd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
+// Plain (coherent) load of a vector entry. The launches of a composed plan are
+// resident before their predecessors have written (they trigger their
+// dependents at their start), and so is the launch after the last one: every
+// kernel that can follow one reads vectors through this, never through the
+// read-only path, which is for data that nothing writes while the kernel is
+// resident.
+template <class T>
+__device__ __forceinline__ T ldv(const T* p);
+template <>
+__device__ __forceinline__ double ldv<double>(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+template <>
+__device__ __forceinline__ float ldv<float>(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+template <>
+__device__ __forceinline__ double2 ldv<double2>(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
 // y = A x  (or y = f - A x when f != null). LPR lanes cooperate on one row and
 // reduce with shuffles; rows of a 7-point stencil use 8 lanes.
 template <class T, int LPR>
 __global__ void __launch_bounds__(256) k_spmv(uint32_t n, const uint32_t* __restrict__ ia,
                                               const uint32_t* __restrict__ ja, const T* __restrict__ a,
-                                              const T* __restrict__ x, T* __restrict__ y,
-                                              const T* __restrict__ f) {
+                                              const T* x, T* __restrict__ y, const T* f) {
     pdl_wait();
     pdl_trigger();
     uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,11 +95,11 @@ __global__ void __launch_bounds__(256) k_spmv(uint32_t n, const uint32_t* __rest
     T s = 0;
     if (active) {
         uint32_t e = ia[row + 1];
-        for (uint32_t j = ia[row] + lane; j < e; j += LPR) s = fmadd(a[j], x[ja[j]], s);
+        for (uint32_t j = ia[row] + lane; j < e; j += LPR) s = fmadd(a[j], ldv(x + ja[j]), s);
     }
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (active && lane == 0) y[row] = f ? f[row] - s : s;
+    if (active && lane == 0) y[row] = f ? ldv(f + row) - s : s;
 }
 
 // Staged CSR SpMV: a CTA takes tiles of ST_ROWS consecutive rows; the tile's
@@ -193,8 +219,8 @@ __device__ __forceinline__ void spmv_pipe_v(uint32_t n, const uint32_t* __restri
 
 template <class T, bool SA, class Epi>
 __device__ __forceinline__ void spmv_pipe(uint32_t n, const uint32_t* __restrict__ ia, const uint32_t* __restrict__ ja,
-                                          const T* __restrict__ a, const T* __restrict__ x, uint32_t cap, Epi epi) {
-    spmv_pipe_v<T, SA>(n, ia, ja, a, [&](uint32_t c) { return x[c]; }, cap, epi);
+                                          const T* __restrict__ a, const T* x, uint32_t cap, Epi epi) {
+    spmv_pipe_v<T, SA>(n, ia, ja, a, [&](uint32_t c) { return ldv(x + c); }, cap, epi);
 }
 
 // ---- sliced rows ----------------------------------------------------------
@@ -245,7 +271,7 @@ __device__ __forceinline__ void sell_rows(uint32_t n, const uint32_t* __restrict
         for (uint32_t k0 = 0;;) {
             double xv[SELL_K];
 #pragma unroll
-            for (int k = 0; k < SELL_K; k++) xv[k] = c[k] != SELL_NONE ? x[c[k]] : 0.0;
+            for (int k = 0; k < SELL_K; k++) xv[k] = c[k] != SELL_NONE ? ldv(x + c[k]) : 0.0;
 #pragma unroll
             for (int k = 0; k < SELL_K; k++)
                 if (c[k] != SELL_NONE) s = fmadd(v[k], xv[k], s);
@@ -263,9 +289,9 @@ __device__ __forceinline__ void sell_rows(uint32_t n, const uint32_t* __restrict
 template <int MODE>  // 0: y = A x, 1: y = f - A x
 __global__ void __launch_bounds__(256, 4) k_spmv_sell(uint32_t n, const uint32_t* __restrict__ soff,
                                                       const uint32_t* __restrict__ scol,
-                                                      const double* __restrict__ sval, const double* __restrict__ x,
-                                                      double* __restrict__ y, const double* __restrict__ f) {
-    sell_rows(n, soff, scol, sval, x, [&](uint32_t row, double s) { y[row] = MODE ? f[row] - s : s; });
+                                                      const double* __restrict__ sval, const double* x,
+                                                      double* __restrict__ y, const double* f) {
+    sell_rows(n, soff, scol, sval, x, [&](uint32_t row, double s) { y[row] = MODE ? ldv(f + row) - s : s; });
 }
 // one wave of four CTAs an SM
 static unsigned sell_grid(uint32_t n) {
@@ -353,9 +379,8 @@ __global__ void __launch_bounds__(ST_ROWS) k_update_staged(uint32_t N, const uin
 template <class T, int MODE, bool SA>  // MODE 0: y = A x, 1: y = f - A x
 __global__ void __launch_bounds__(ST_ROWS) k_spmv_staged(uint32_t n, const uint32_t* __restrict__ ia,
                                                          const uint32_t* __restrict__ ja, const T* __restrict__ a,
-                                                         const T* __restrict__ x, T* __restrict__ y,
-                                                         const T* __restrict__ f, uint32_t cap) {
-    spmv_pipe<T, SA>(n, ia, ja, a, x, cap, [&](uint32_t row, T acc) { y[row] = MODE ? f[row] - acc : acc; });
+                                                         const T* x, T* __restrict__ y, const T* f, uint32_t cap) {
+    spmv_pipe<T, SA>(n, ia, ja, a, x, cap, [&](uint32_t row, T acc) { y[row] = MODE ? ldv(f + row) - acc : acc; });
 }
 
 __global__ void k_tile_max(uint32_t n, const uint32_t* __restrict__ ia, uint32_t* __restrict__ out) {
@@ -636,23 +661,6 @@ __global__ void k_chebk(uint32_t n, T* __restrict__ x2, const T* __restrict__ u1
     }
 }
 
-// Plain (coherent) load of a vector entry that an earlier launch of the chain
-// wrote; see the composed sweeps.
-template <class T>
-__device__ __forceinline__ T ldv(const T* p);
-template <>
-__device__ __forceinline__ double ldv<double>(const double* p) {
-    double v;
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-template <>
-__device__ __forceinline__ float ldv<float>(const float* p) {
-    float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 // Dense coarsest level: x = C^{-1} f, one warp per row. The operator's type
 // CT may be wider than the vectors' T: the FP32 hierarchy keeps its coarsest
 // solve (the dense inverse, or the tabulated small-level operator standing in
@@ -771,19 +779,24 @@ __global__ void k_to_f64(uint32_t n, const float* __restrict__ a, double* __rest
     if (i < n) b[i] = (double)a[i];
 }
 // dst = src[idx] and dst[idx] = src; `ahead`: between the launches of a plan,
-// as programmatic dependent launches like theirs.
+// as programmatic dependent launches like those of a step plan, which follows
+// the gather: the dependents are let in after the wait.
 __global__ void k_gather(uint32_t n, const uint32_t* __restrict__ idx, const double* src, double* __restrict__ dst,
                          int ahead) {
-    if (ahead) pdl_trigger();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = i < n ? idx[i] : 0;
-    if (ahead) pdl_wait();
+    if (ahead) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (i < n) dst[i] = ldv(src + j);
 }
 __global__ void k_scatter(uint32_t n, const uint32_t* __restrict__ idx, const double* src, double* __restrict__ dst,
                           int ahead) {
-    if (ahead) pdl_trigger();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = i < n ? idx[i] : 0;
-    if (ahead) pdl_wait();
+    if (ahead) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (i < n) dst[j] = ldv(src + i);
 }
 __global__ void k_relabel(uint32_t n, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ map,
@@ -1264,8 +1277,7 @@ __global__ void __launch_bounds__(256, merge_a_min_ctas<T>()) k_merge_a(uint32_t
 // in registers, and what a launch adds to the chain is its wait, one round of
 // gathers and its store. Until its wait returns a kernel may touch constants
 // only (the launches before its predecessor may still run), and vectors are
-// read with plain loads: the read-only path is for data that no kernel writes
-// while this one is resident.
+// read with plain loads (ldv).
 // ClassedRows as a kernel takes them; block0[c]: first block of class c.
 template <class T>
 struct RowSet {
@@ -1775,7 +1787,18 @@ struct Builder {
         ~LevelScope() { r = saved; }
     };
 
+    // The next launch follows a composed one, whose dependents are resident while
+    // it writes, and reads its vectors through the read-only path: without a
+    // programmatic dependent launch.
+    bool plain_next = false;
     void op(std::function<void(cudaStream_t)> f, const char* name = "op") {
+        if (plain_next) {
+            plain_next = false;
+            f = [g = std::move(f)](cudaStream_t s) {
+                PdlOff plain;
+                g(s);
+            };
+        }
         plan.ops.push_back(std::move(f));
         plan.names.push_back(std::string(name) + " L" + std::to_string(cur_level));
         plan.bytes_start.push_back(bytes);
@@ -2360,6 +2383,7 @@ struct Builder {
         const double* C = so->coarse.p;
         uint32_t n = H.lv[j]->n;
         if (!C && !dense_next(j, C, n)) {
+            plain_next = true;
             ms(j + 1, wc, y);
             return;
         }
@@ -3159,7 +3183,7 @@ __device__ __forceinline__ void leave_partials(double part, double* partials, Pc
 template <int LPR>
 __global__ void __launch_bounds__(RB) k_pcg_spmv_dot(uint32_t n, const uint32_t* __restrict__ ia,
                                                      const uint32_t* __restrict__ ja, const double* __restrict__ a,
-                                                     const double* __restrict__ p, double* __restrict__ Ap,
+                                                     const double* p, double* __restrict__ Ap,
                                                      double* partials, PcgDev* d) {
     pdl_wait();
     pdl_trigger();
@@ -3172,13 +3196,13 @@ __global__ void __launch_bounds__(RB) k_pcg_spmv_dot(uint32_t n, const uint32_t*
         double s = 0;
         if (active) {
             uint32_t e = ia[row + 1];
-            for (uint32_t j = ia[row] + lane; j < e; j += LPR) s += a[j] * p[ja[j]];
+            for (uint32_t j = ia[row] + lane; j < e; j += LPR) s += a[j] * ldv(p + ja[j]);
         }
 #pragma unroll
         for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (active && lane == 0) {
             Ap[row] = s;
-            part += s * p[row];
+            part += s * ldv(p + row);
         }
     }
     leave_partials(part, partials, d);
@@ -3188,14 +3212,13 @@ __global__ void __launch_bounds__(RB) k_pcg_spmv_dot(uint32_t n, const uint32_t*
 template <bool SA>
 __global__ void __launch_bounds__(ST_ROWS) k_pcg_spmv_dot_staged(uint32_t n, const uint32_t* __restrict__ ia,
                                                                  const uint32_t* __restrict__ ja,
-                                                                 const double* __restrict__ a,
-                                                                 const double* __restrict__ p,
+                                                                 const double* __restrict__ a, const double* p,
                                                                  double* __restrict__ Ap, double* partials,
                                                                  PcgDev* d, uint32_t cap) {
     double part = 0;
     spmv_pipe<double, SA>(n, ia, ja, a, p, cap, [&](uint32_t row, double acc) {
         Ap[row] = acc;
-        part += acc * p[row];
+        part += acc * ldv(p + row);
     });
     leave_partials(part, partials, d);
 }
@@ -3208,7 +3231,7 @@ __global__ void __launch_bounds__(ST_ROWS, 4) k_pcg_spmv_dot_sell(uint32_t n, co
     double part = 0;
     sell_rows(n, soff, scol, sval, p, [&](uint32_t row, double s) {
         Ap[row] = s;
-        part += s * p[row];
+        part += s * ldv(p + row);
     });
     leave_partials(part, partials, d);
 }
@@ -3264,7 +3287,7 @@ static void launch_pcg_spmv_dot_staged(uint32_t n, const DCSR& Af, const double*
 // it and keeps the loop going while ||r||/||r0|| > eps (pcg.cc:42), no error
 // was flagged and the cap is not hit.
 __global__ void __launch_bounds__(RB) k_pcg_update(uint32_t n, double* __restrict__ x, double* __restrict__ r,
-                                                   const double* __restrict__ p, const double* __restrict__ Ap,
+                                                   const double* __restrict__ p, const double* Ap,
                                                    const double* spmv_partials, double* partials, PcgDev* d,
                                                    cudaGraphConditionalHandle h, int cond) {
     pdl_wait();
@@ -3290,7 +3313,7 @@ __global__ void __launch_bounds__(RB) k_pcg_update(uint32_t n, double* __restric
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 const uint32_t j = i + k * stride;
-                if (j < n2) { xv[k] = x2[j]; pv[k] = p2[j]; rv[k] = r2[j]; av[k] = a2[j]; }
+                if (j < n2) { xv[k] = x2[j]; pv[k] = p2[j]; rv[k] = r2[j]; av[k] = ldv(a2 + j); }
             }
         };
         uint32_t i = t0;
@@ -3312,7 +3335,7 @@ __global__ void __launch_bounds__(RB) k_pcg_update(uint32_t n, double* __restric
         if ((n & 1) && t0 == 0) {
             const uint32_t i = n - 1;
             x[i] += alpha * p[i];
-            double ri = r[i] - alpha * Ap[i];
+            double ri = r[i] - alpha * ldv(Ap + i);
             r[i] = ri;
             part += ri * ri;
         }
@@ -3320,7 +3343,7 @@ __global__ void __launch_bounds__(RB) k_pcg_update(uint32_t n, double* __restric
         scalars();
         for (uint32_t i = t0; i < n; i += stride) {
             x[i] += alpha * p[i];
-            double ri = r[i] - alpha * Ap[i];
+            double ri = r[i] - alpha * ldv(Ap + i);
             r[i] = ri;
             part += ri * ri;
         }
@@ -3343,8 +3366,7 @@ __global__ void __launch_bounds__(RB) k_pcg_update(uint32_t n, double* __restric
 }
 
 // Partial sums of (r, z) and, for the flexible beta, (Ap, z).
-__global__ void __launch_bounds__(RB) k_pcg_dot_rz(uint32_t n, const double* __restrict__ r,
-                                                   const double* __restrict__ z, const double* __restrict__ Ap,
+__global__ void __launch_bounds__(RB) k_pcg_dot_rz(uint32_t n, const double* r, const double* z, const double* Ap,
                                                    double* partials, PcgDev* d, int flexible) {
     pdl_wait();
     pdl_trigger();
@@ -3356,21 +3378,22 @@ __global__ void __launch_bounds__(RB) k_pcg_dot_rz(uint32_t n, const double* __r
         const double2* q2 = reinterpret_cast<const double2*>(Ap);
         const uint32_t n2 = n >> 1;
         for (uint32_t i = t0; i < n2; i += stride) {
-            double2 rv = r2[i], zv = z2[i];
+            double2 rv = ldv(r2 + i), zv = ldv(z2 + i);
             part += rv.x * zv.x; part += rv.y * zv.y;
             if (flexible) {
-                double2 qv = q2[i];
+                double2 qv = ldv(q2 + i);
                 part2 += qv.x * zv.x; part2 += qv.y * zv.y;
             }
         }
         if ((n & 1) && t0 == 0) {
-            part += r[n - 1] * z[n - 1];
-            if (flexible) part2 += Ap[n - 1] * z[n - 1];
+            part += ldv(r + n - 1) * ldv(z + n - 1);
+            if (flexible) part2 += ldv(Ap + n - 1) * ldv(z + n - 1);
         }
     } else {
         for (uint32_t i = t0; i < n; i += stride) {
-            part += r[i] * z[i];
-            if (flexible) part2 += Ap[i] * z[i];
+            const double zv = ldv(z + i);
+            part += ldv(r + i) * zv;
+            if (flexible) part2 += ldv(Ap + i) * zv;
         }
     }
     part = block_sum(part);
