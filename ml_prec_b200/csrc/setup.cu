@@ -477,18 +477,20 @@ struct RowTable {
         full = false;
         sync();
     }
-    __device__ __forceinline__ void add(uint32_t c, double v) {
-        if (full) return;  // the row is lost already
+    // whether the column is a new one
+    __device__ __forceinline__ bool add(uint32_t c, double v) {
+        if (full) return true;  // the row is lost already
         uint32_t h = (c * 2654435761u) >> 16;
         for (uint32_t p = 0; p < size; p++) {
             const uint32_t t = (h + p) & (size - 1);
             const uint32_t k = atomicCAS(&key[t], EMPTY, c);
             if (k == EMPTY || k == c) {
                 val[t] += v;
-                return;
+                return k == EMPTY;
             }
         }
         full = true;
+        return true;
     }
     // adds coef * (entries [b, e) of col, v); the lanes meet
     __device__ __forceinline__ void add_row(const uint32_t* col, const double* v, uint32_t b, uint32_t e, double coef) {
@@ -547,7 +549,8 @@ struct RowTable {
 // Each permuted row i < N-Md is processed by a group of lanes (or, when it
 // outgrows their table, by one thread) and ends in its own slot of `cap`
 // (column, value) pairs sorted by column. The row is loaded as the
-// diagonal aux[map[i]] minus the kept links scaled by 1/beta (ja order), then
+// diagonal aux[map[i]] minus the kept links scaled by 1/beta (ja order; links
+// that repeat a column are added up, so that a row's columns differ), then
 // the slot's columns k < min(i, M) are eliminated in increasing order with
 // l_ik = w_k / U_kk and the k-th U row's updates, fill allowed. l_ik overwrites
 // the value of column k; after the loop the slot holds the L entries first and
@@ -593,6 +596,7 @@ __device__ int lu_row(const LUArgs& g, uint32_t i, int round) {
     uint32_t wn = 1;
     wc[0] = i;
     double diag = g.aux[arow];
+    wv[0] = -0.0;  // links to the row itself
     for (uint32_t j_ = g.Aia[arow] + 1; j_ < g.Aia[arow + 1]; j_++) {
         if (!g.keep[j_]) continue;
         uint32_t nj = g.rmap[g.Aja[j_]];
@@ -600,11 +604,16 @@ __device__ int lu_row(const LUArgs& g, uint32_t i, int round) {
         if (wn == cap) return -1;
         uint32_t p = wn;
         while (p > 0 && wc[p - 1] > nj) { wc[p] = wc[p - 1]; wv[p] = wv[p - 1]; p--; }
-        wc[p] = nj; wv[p] = z; wn++;
+        if (p > 0 && wc[p - 1] == nj) {
+            wv[p - 1] += z;
+            for (; p < wn; p++) { wc[p] = wc[p + 1]; wv[p] = wv[p + 1]; }  // close the gap
+        } else {
+            wc[p] = nj; wv[p] = z; wn++;
+        }
         diag -= z;
     }
     for (uint32_t t = 0; t < wn; t++)
-        if (wc[t] == i) { wv[t] = diag; break; }
+        if (wc[t] == i) { wv[t] += diag; break; }
     uint32_t m = i < g.M ? i : g.M;
     uint32_t t = 0;
     for (; t < wn && wc[t] < m; t++) {
@@ -654,7 +663,9 @@ __device__ int lu_row(const LUArgs& g, uint32_t i, int round, RowTable<W, CAP>& 
         if (j < re && g.keep[j]) {
             const uint32_t c = g.rmap[g.Aja[j]];
             z = g.Aa[j] / g.beta;
-            t.add(c, z);
+            // lanes that hold one column would add to it at the same time: such a
+            // row is left to one thread
+            if (c == i || !t.add(c, z)) t.full = true;
             if (c < m && !g.ready(c, round)) stop = min(stop, c);
         }
         for (uint32_t l = 0; l < W && l < re - b; l++) diag -= __shfl_sync(t.mask, z, l, W);  // in the row's order
@@ -1037,7 +1048,7 @@ __global__ void k_dense_from_csr(uint32_t n, const uint32_t* __restrict__ ia, co
                                  const double* __restrict__ a, double* __restrict__ D) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    for (uint32_t j = ia[i]; j < ia[i + 1]; j++) D[(size_t)i * n + ja[j]] = a[j];
+    for (uint32_t j = ia[i]; j < ia[i + 1]; j++) D[(size_t)i * n + ja[j]] += a[j];
 }
 // Blocked, in place: for the GJ_B pivots from k0 on, the pivot block is inverted
 // by one CTA (P), the block's rows become P times themselves (P itself in the
