@@ -34,6 +34,10 @@ struct Error : std::runtime_error {
     int code;
     Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
+// Device memory ran out: what is optional is left out (build_state, sell_build).
+struct OutOfMemory : Error {
+    using Error::Error;
+};
 
 #define MLP_THROW(code, msg)                                                     \
     do {                                                                         \
@@ -127,6 +131,13 @@ struct DBuf {
 // serialised; Tmp<T> buffers created inside a scope come from the arena, outside
 // one they fall back to the buffer pool.
 void* arena_take(size_t bytes);  // null when no scope is active
+// The arena's state; give_back() returns to it: memory taken since then is free
+// again (its buffers must be gone), chunks allocated since then are released.
+struct ArenaMark {
+    ArenaMark();
+    void give_back(cudaStream_t s);
+    std::vector<size_t> off;
+};
 struct ArenaScope {
     ArenaScope();
     ~ArenaScope();

@@ -322,8 +322,18 @@ __global__ void k_sell_fill(uint32_t n, const uint32_t* __restrict__ ia, const u
         sval[at] = k < l ? a[b + k] : 0.0;
     }
 }
+static void sell_fill(DCSR& m, cudaStream_t s);
 void sell_build(DCSR& m, cudaStream_t s) {
     if (m.nrow < 4 * ST_ROWS) return;
+    try {
+        sell_fill(m, s);
+    } catch (const OutOfMemory&) {  // the matrix stays CSR only
+        m.soff.release();
+        m.scol.release();
+        m.sval.release();
+    }
+}
+static void sell_fill(DCSR& m, cudaStream_t s) {
     const uint32_t nsl = (m.nrow + 31) / 32;
     Tmp<uint32_t> w((size_t)nsl + 1), widest(1);
     widest.zero(s);
@@ -2434,12 +2444,9 @@ struct Builder {
         }
     }
 
-    // The whole application z = B f in composed form (f and z FP64, in frame
-    // order); false, and nothing recorded, where it does not apply.
-    bool state_apply(const double* f, double* z, std::unique_ptr<StateOps>& ops, StateVecs<T>& vecs) {
-        const int systems = state_systems();
-        if (systems < 0) return false;
-        const uint32_t m = (uint32_t)systems;
+    // Operators and vectors of the composed form with m systems; false where it
+    // does not apply.
+    bool state_make(uint32_t m, std::unique_ptr<StateOps>& ops, StateVecs<T>& vecs) {
         const double* C = nullptr;
         uint32_t cn = 0;
         DBuf<double> table;
@@ -2466,6 +2473,35 @@ struct Builder {
             const uint32_t n = H.lv[j]->n ? H.lv[j]->n : 1;
             vecs.u[j - 1].alloc(n);
             if (H.kind == PREC_CHEB) vecs.u2[j - 1].alloc(n);
+        }
+        // P's columns and G's rows in natural order
+        const uint32_t R = H.lv[0]->N - H.lv[0]->Md, *map = H.lv[0]->phi.p;
+        ops->Pcol.alloc(ops->P.m.nnz + 1);
+        ops->Grow.alloc(R + 1);
+        k_relabel<<<grid_for(ops->P.m.nnz, 256), 256, 0, stream>>>(ops->P.m.nnz, ops->P.m.ja.p, map, ops->Pcol.p);
+        k_relabel<<<grid_for(R, 256), 256, 0, stream>>>(R, ops->G.row.p, map, ops->Grow.p);
+        CK_LAUNCH();
+        return true;
+    }
+
+    // The whole application z = B f in composed form (f and z FP64, in frame
+    // order); false, and nothing recorded, where it does not apply or the device
+    // has no memory left for it: the step plan needs none of it.
+    bool state_apply(const double* f, double* z, std::unique_ptr<StateOps>& ops, StateVecs<T>& vecs) {
+        const int systems = state_systems();
+        if (systems < 0) return false;
+        const uint32_t m = (uint32_t)systems;
+        ArenaMark mark;
+        bool made = false;
+        try {
+            made = state_make(m, ops, vecs);
+        } catch (const OutOfMemory&) {
+        }
+        if (!made) {
+            ops.reset();
+            vecs = StateVecs<T>();
+            mark.give_back(stream);
+            return false;
         }
         so = ops.get();
         sv = &vecs;
@@ -2499,12 +2535,7 @@ struct Builder {
         }, "phase2_folded");
         bytes += rowset_bytes(ops->G) + 8ull * ops->G.first[1] * dn + (sizeof(T) + 8ull) * R;
         // the same two launches on natural-order vectors
-        ops->Pcol.alloc(ops->P.m.nnz + 1);
-        ops->Grow.alloc(R + 1);
         const uint32_t* map = L.phi.p;
-        k_relabel<<<grid_for(ops->P.m.nnz, 256), 256, 0, stream>>>(ops->P.m.nnz, Ps.ja, map, ops->Pcol.p);
-        k_relabel<<<grid_for(R, 256), 256, 0, stream>>>(R, Gs.row, map, ops->Grow.p);
-        CK_LAUNCH();
         RowSet<T> Pn = Ps, Gn = Gs;
         Pn.ja = ops->Pcol.p;
         Gn.row = ops->Grow.p;

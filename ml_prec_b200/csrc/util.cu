@@ -57,6 +57,8 @@ void trace_flush() {
 }
 
 // ---- scratch arena ----------------------------------------------------------
+static void* device_alloc(size_t bytes);
+
 namespace {
 struct DevArena {
     std::mutex mu;
@@ -107,10 +109,25 @@ void* arena_take(size_t bytes) {
             return p;
         }
     size_t cap = std::max<size_t>(bytes, (size_t)64 << 20);
-    char* base = nullptr;
-    CK(cudaMalloc(&base, cap));
+    char* base = static_cast<char*>(device_alloc(cap));
     a->chunks.push_back({base, cap, bytes});
     return base;
+}
+
+ArenaMark::ArenaMark() {
+    if (!t_arena) return;
+    for (auto& c : t_arena->chunks) off.push_back(c.off);
+}
+
+void ArenaMark::give_back(cudaStream_t s) {
+    CK(cudaStreamSynchronize(s));
+    if (!t_arena) return;
+    auto& chunks = t_arena->chunks;
+    while (chunks.size() > off.size()) {
+        cudaFree(chunks.back().base);
+        chunks.pop_back();
+    }
+    for (size_t i = 0; i < off.size(); i++) chunks[i].off = off[i];
 }
 
 // ---- device buffer pool -------------------------------------------------------
@@ -215,6 +232,34 @@ void d2h_large(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     }
 }
 
+// cudaMalloc; when the device is out of memory, once more after the pool's cached
+// blocks are given back.
+static void* device_alloc(size_t bytes) {
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        int dev = 0;
+        cudaGetLastError();
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceSynchronize());
+        Pool& P = pool();
+        {
+            std::lock_guard<std::mutex> lk(P.mu);
+            for (void* q : P.pending[dev]) { P.free_[dev].emplace(P.live[q].bytes, q); P.live.erase(q); }
+            P.pending[dev].clear();
+            for (auto& kv : P.free_[dev]) cudaFree(kv.second);
+            P.free_[dev].clear();
+        }
+        e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            throw OutOfMemory(ERR_CUDA, "cudaMalloc of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
+        }
+    }
+    CK(e);
+    return p;
+}
+
 void* pool_alloc(size_t bytes) {
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -231,21 +276,7 @@ void* pool_alloc(size_t bytes) {
             return p;
         }
     }
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, cls);
-    if (e != cudaSuccess) {
-        // out of memory: give the cached blocks back and try once more
-        cudaGetLastError();
-        CK(cudaDeviceSynchronize());
-        {
-            std::lock_guard<std::mutex> lk(P.mu);
-            for (void* q : P.pending[dev]) { P.free_[dev].emplace(P.live[q].bytes, q); P.live.erase(q); }
-            P.pending[dev].clear();
-            for (auto& kv : P.free_[dev]) cudaFree(kv.second);
-            P.free_[dev].clear();
-        }
-        CK(cudaMalloc(&p, cls));
-    }
+    void* p = device_alloc(cls);
     std::lock_guard<std::mutex> lk(P.mu);
     P.live[p] = {dev, cls, false};
     return p;
