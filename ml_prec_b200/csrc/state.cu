@@ -400,7 +400,7 @@ std::unique_ptr<StateOps> build_state(const Hierarchy& H, uint32_t m, const doub
                                       cudaStream_t s) {
     auto S = std::unique_ptr<StateOps>(new StateOps());
     S->m = m;
-    S->whole = C && cn <= ABSORB_WHOLE;
+    S->whole = C && cn <= ABSORB_WHOLE && !fp32;
     S->absorbed = S->whole;
     S->K.resize(m);
     Builder B(s, fp32);

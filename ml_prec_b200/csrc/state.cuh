@@ -49,7 +49,7 @@ struct StateOps {
     uint32_t m = 0;         // systems 1..m have a K
     bool absorbed = false;  // system m's sweeps need no coarse call: its coarse operator is part
                             // of K (absorbed whole, or as the dense part of K's class 0)
-    bool whole = false;     // absorbed in G as well: the state's C entries stay w_C to the end
+    bool whole = false;     // absorbed in G as well (FP64): the state's C entries stay w_C to the end
     ClassedRows P;          // rows [0, R0): [w_E0; v0 of system 1] = P f
     ClassedRows G;          // rows [0, R0), columns [0, R0): x = G [w_E0; state of system 1]
     std::vector<ClassedRows> K;  // K[j - 1]: the N_j rows of system j, in its frame
@@ -60,7 +60,9 @@ struct StateOps {
 // Builds the operators of systems 1..m of H (levels 1..m must not be direct and
 // must hold their dropped-link values). C (cn x cn, row-major, FP64) is the
 // dense operator of level m + 1, or null. Up to ABSORB_WHOLE rows it becomes
-// part of K_m and G as any other factor. Larger, K_m's rows with coarse
+// part of K_m and G as any other factor; not in an FP32 hierarchy, whose coarse
+// solve keeps FP64 entries and sums (60x220x20 iid, 4 coarse rows: one launch
+// more, 24.5 us an application in place of 23). Larger, K_m's rows with coarse
 // columns (nd of them) take their product with it as a dense part, K_C C,
 // where that is at most ABSORB_DENSE bytes: a sweep then reads nd x cn entries
 // but needs no coarse launch (without a system, m = 0, G's rows do). At level 2 of the 60x220x85 field (cn = 422, nd =
