@@ -75,8 +75,10 @@ typedef struct {
     const uint32_t* ncheb;
     int32_t fp32;            /* 1: store and apply the hierarchy in FP32              */
     int32_t autotune;        /* 1: time the row kernels' launch shapes (lanes per row,
-                                block size) on each level at build and keep the
-                                fastest (cached per level shape); 0: fixed heuristic */
+                                block size) on each level at build, take the fastest
+                                (cached per level shape) and keep the plan of these
+                                steps where it is faster than the composed one
+                                (cached per hierarchy shape); 0: no timing          */
     uint32_t neps;           /* multi-split inner_iter = dynamic (msplit.cfg level_eps,
                                 multi_split_constr.cc:198-203, 256-264): per-level eps,
                                 entry 0 ignored, last value repeats; each level call

@@ -1533,7 +1533,8 @@ static uint32_t spmv_lpr(uint32_t n, uint32_t nnz, uint32_t tile_max) {
 // equal-shaped members, or a rebuild, tunes once. Without it the shape is the
 // fixed heuristic (pick_lpr lanes, 256 threads). The lane count changes the
 // order in which a row's products are added, so tuned and untuned plans agree
-// to rounding.
+// to rounding. The tuned step plan is then timed against the composed plan,
+// where that applies, and the faster one kept (record_plan).
 // ---------------------------------------------------------------------------
 struct LaunchShape {
     int lpr = 1;
@@ -1543,6 +1544,7 @@ struct LaunchShape {
 namespace {
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, uint32_t, uint32_t>, LaunchShape> g_tune;
+std::map<std::vector<uint32_t>, bool> g_tune_composed;  // by the hierarchy's shape: the composed plan is faster
 }  // namespace
 
 template <class Launch>
@@ -2872,6 +2874,82 @@ static cudaGraph_t capture(cudaStream_t s, F&& launches) {
     return g;
 }
 
+// Device time of a plan's launches, the best of a few.
+static float plan_time(const Plan& plan, cudaStream_t s) {
+    cudaEvent_t e0, e1;
+    CK(cudaEventCreate(&e0));
+    CK(cudaEventCreate(&e1));
+    float best = 1e30f;
+    for (int r = 0; r < 4; r++) {  // the first one warms up
+        CK(cudaEventRecord(e0, s));
+        plan.run(s);
+        CK(cudaEventRecord(e1, s));
+        CK(cudaEventSynchronize(e1));
+        CK(cudaGetLastError());
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, e0, e1));
+        if (r && ms < best) best = ms;
+    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    return best;
+}
+
+// Records the application: the composed form where it applies, else the step
+// plan (steps). With autotune both are made and timed, and the choice is
+// remembered by the hierarchy's shape like the launch shapes are.
+template <class T, class Make, class Steps>
+static void record_plan(Prec& P, StateVecs<T>& vecs, bool autotune, cudaStream_t s, Make make, Steps steps) {
+    Hierarchy& H = *P.H;
+    Builder<T> B = make(P.plan);
+    std::vector<uint32_t> shape{(uint32_t)sizeof(T), (uint32_t)H.kind};
+    for (uint32_t l = 0; l < H.nlevels; l++) {
+        const Level& L = *H.lv[l];
+        shape.insert(shape.end(), {L.N, L.nnz, L.M, L.Md, L.niter, L.ncheb});
+    }
+    bool known = false, composed = true;
+    if (autotune) {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tune_composed.find(shape);
+        known = it != g_tune_composed.end();
+        if (known) composed = it->second;
+    }
+    composed = composed && B.state_apply(P.fin, P.fout, P.state, vecs);
+    Builder<T>* kept = &B;
+    Plan tuned;
+    Builder<T> S = make(tuned);
+    if (!composed) {
+        steps(B);
+    } else if (autotune && !known) {
+        float tc = plan_time(P.plan, s), ts = 1e30f;
+        try {
+            steps(S);
+            ts = plan_time(tuned, s);
+        } catch (const OutOfMemory&) {  // no candidate then, nor is one of too many steps
+        } catch (const Error& e) {
+            if (e.code != ERR_LIMIT) throw;
+        }
+        composed = tc <= ts;
+        trace(("autotune: composed " + std::to_string(1e3f * tc) + " us, steps " + std::to_string(1e3f * ts) + " us").c_str());
+        if (!composed) {
+            P.plan = std::move(tuned);
+            P.state.reset();
+            vecs = StateVecs<T>();
+            kept = &S;
+        }
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        g_tune_composed[shape] = composed;
+    }
+    if (composed) {
+        P.first_natural = B.first_natural;
+        P.last_natural = B.last_natural;
+    }
+    P.bytes_per_apply = kept->bytes + (composed || sizeof(T) == 8 ? 0 : 12ull * H.lv[0]->N * 2);
+    P.plan.bytes_total = kept->bytes;
+    P.persist_regions = kept->persist_regions;
+    P.persist_steps = kept->persist_steps;
+}
+
 std::unique_ptr<Prec> make_prec(const DCSR& A, const BuildCfg& cfg, bool fp32, cudaStream_t s) {
     ArenaScope arena;
     auto P = std::unique_ptr<Prec>(new Prec());
@@ -2898,20 +2976,18 @@ std::unique_ptr<Prec> make_prec(const DCSR& A, const BuildCfg& cfg, bool fp32, c
         alloc_work<double>(H, P->w64);
         P->sp64.reset(new SmallPlan<double>());
         if (small_budget() && !dyn) build_small<double>(H, *P->sp64, small_budget(), s);
-        Builder<double> B{H, P->w64, P->plan, P->sp64.get()};
-        B.explicit_solves = explicit_solves;
-        B.stream = s;
-        B.autotune = cfg.autotune != 0;
-        builder_persist(B, *P);
-        if (B.state_apply(P->fin, P->fout, P->state, P->sv64)) {}
-        else if (H.kind == PREC_MSPLIT) B.ms(0, P->fin, P->fout);
-        else B.ch(0, P->fin, P->fout);
-        P->bytes_per_apply = B.bytes;
-        P->plan.bytes_total = B.bytes;
-        P->first_natural = B.first_natural;
-        P->last_natural = B.last_natural;
-        P->persist_regions = B.persist_regions;
-        P->persist_steps = B.persist_steps;
+        auto make = [&](Plan& plan) {
+            Builder<double> B{H, P->w64, plan, P->sp64.get()};
+            B.explicit_solves = explicit_solves;
+            B.stream = s;
+            B.autotune = cfg.autotune != 0;
+            builder_persist(B, *P);
+            return B;
+        };
+        record_plan<double>(*P, P->sv64, cfg.autotune != 0, s, make, [&](Builder<double>& B) {
+            if (H.kind == PREC_MSPLIT) B.ms(0, P->fin, P->fout);
+            else B.ch(0, P->fin, P->fout);
+        });
     } else {
         for (uint32_t l = 0; l < H.nlevels; l++) {
             Level& L = *H.lv[l];
@@ -2939,34 +3015,31 @@ std::unique_ptr<Prec> make_prec(const DCSR& A, const BuildCfg& cfg, bool fp32, c
         }
         P->f32.alloc(N0);
         P->z32.alloc(N0);
-        Builder<float> B{H, P->w32, P->plan, P->sp32.get()};
-        B.small64 = P->sp64.get();
-        B.explicit_solves = explicit_solves;
-        B.stream = s;
-        B.autotune = cfg.autotune != 0;
-        builder_persist(B, *P);
+        auto make = [&](Plan& plan) {
+            Builder<float> B{H, P->w32, plan, P->sp32.get()};
+            B.small64 = P->sp64.get();
+            B.explicit_solves = explicit_solves;
+            B.stream = s;
+            B.autotune = cfg.autotune != 0;
+            builder_persist(B, *P);
+            return B;
+        };
         const double* fin = P->fin;
         float* f32 = P->f32.p;
         float* z32 = P->z32.p;
         double* fout = P->fout;
-        auto top = [&] {
-            if (B.ps) B.ps->push_back(Builder<float>::pstep(PS_TOF32, 1, N0, 0, nullptr, nullptr, nullptr, nullptr, fin, f32));
-            else B.op([=](cudaStream_t st) { launch_k(k_to_f32, grid_for(N0, 256), 256, 0, st, N0, fin, f32); }, "to_f32");
-            if (H.kind == PREC_MSPLIT) B.ms(0, f32, z32);
-            else B.ch(0, f32, z32);
-            if (B.ps) B.ps->push_back(Builder<float>::pstep(PS_TOF64, 1, N0, 0, nullptr, nullptr, nullptr, nullptr, z32, fout));
-            else B.op([=](cudaStream_t st) { launch_k(k_to_f64, grid_for(N0, 256), 256, 0, st, N0, (const float*)z32, fout); }, "to_f64");
-        };
-        const bool composed = B.state_apply(P->fin, P->fout, P->state, P->sv32);
-        if (composed) {}
-        else if (B.persist_ok(0)) B.persist_region(top);
-        else top();
-        P->bytes_per_apply = B.bytes + (composed ? 0 : 12ull * N0 * 2);
-        P->plan.bytes_total = B.bytes;
-        P->first_natural = B.first_natural;
-        P->last_natural = B.last_natural;
-        P->persist_regions = B.persist_regions;
-        P->persist_steps = B.persist_steps;
+        record_plan<float>(*P, P->sv32, cfg.autotune != 0, s, make, [&](Builder<float>& B) {
+            auto top = [&] {
+                if (B.ps) B.ps->push_back(Builder<float>::pstep(PS_TOF32, 1, N0, 0, nullptr, nullptr, nullptr, nullptr, fin, f32));
+                else B.op([=](cudaStream_t st) { launch_k(k_to_f32, grid_for(N0, 256), 256, 0, st, N0, fin, f32); }, "to_f32");
+                if (H.kind == PREC_MSPLIT) B.ms(0, f32, z32);
+                else B.ch(0, f32, z32);
+                if (B.ps) B.ps->push_back(Builder<float>::pstep(PS_TOF64, 1, N0, 0, nullptr, nullptr, nullptr, nullptr, z32, fout));
+                else B.op([=](cudaStream_t st) { launch_k(k_to_f64, grid_for(N0, 256), 256, 0, st, N0, (const float*)z32, fout); }, "to_f64");
+            };
+            if (B.persist_ok(0)) B.persist_region(top);
+            else top();
+        });
     }
     sell_build(H.lv[0]->Af, s);
     CK(cudaStreamSynchronize(s));

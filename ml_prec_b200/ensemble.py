@@ -6,9 +6,9 @@ nz in [10, 85] (seeded) and its own i.i.d. log-normal field (the
 small-mesh model), its own matrix and FP32-stored multi-split hierarchy; the forward
 solves (right-hand side from the Dirichlet faces) and the adjoint solves
 (misfit gradient at 25 observation cells) of all realizations each run as one
-graph launch (mlp_ensemble_solve). The members' row kernels take their launch
-shapes from the build-time autotuner (mlp_prec_cfg.autotune). Sharding the
-ensemble over several GPUs
+graph launch (mlp_ensemble_solve). Each member's plan is the faster of the
+composed one and the steps with launch shapes from the build-time autotuner
+(mlp_prec_cfg.autotune). Sharding the ensemble over several GPUs
 assigns whole realizations to ranks (no data exchange during the solves).
 """
 from __future__ import annotations
