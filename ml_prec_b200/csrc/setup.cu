@@ -1050,23 +1050,31 @@ __global__ void k_dense_from_csr(uint32_t n, const uint32_t* __restrict__ ia, co
     if (i >= n) return;
     for (uint32_t j = ia[i]; j < ia[i + 1]; j++) D[(size_t)i * n + ja[j]] += a[j];
 }
-// Blocked, in place: for the GJ_B pivots from k0 on, the pivot block is inverted
-// by one CTA (P), the block's rows become P times themselves (P itself in the
-// block's columns), and every other row i loses D_i,block times them. One pivot
-// at a time it was three launches a pivot, 28 ms for the 1,606 rows of the
-// two-level 60x220x10 problem; blocks of 32 take three launches for
-// 32 pivots (set-up of that problem, hierarchy and all: 35 -> 6 ms). No pivoting.
+// One pivot at a time (three launches each) took 28 ms for the 1,606 rows of the
+// two-level 60x220x10 problem; blocks of 32 pivots take three launches for 32
+// (set-up of that problem, hierarchy and all: 35 -> 3.7 ms). In place and without
+// pivoting; every entry sees the pivots of a block one after another, as it
+// would singly, so the result is the same to the last bit. (With the block's
+// explicit inverse in their place it is not: on a matrix of 40 rows with
+// condition number 1e9 that lost five digits.) One CTA takes the block itself and
+// keeps each pivot's column (Cb) and scaled row (Rb); the panel kernel takes the
+// block's rows and columns outside it through them and keeps theirs (R, C); the
+// update subtracts their products from the rest.
 constexpr uint32_t GJ_B = 32;
 constexpr uint32_t GJ_T = 64;  // rows and columns of an update tile
-__global__ void __launch_bounds__(GJ_B* GJ_B) k_gj_block(uint32_t n, uint32_t k0, uint32_t kb, const double* __restrict__ D,
-                                                         double* __restrict__ P, int* __restrict__ err) {
+__global__ void __launch_bounds__(GJ_B* GJ_B) k_gj_block(uint32_t n, uint32_t k0, uint32_t kb, double* __restrict__ D,
+                                                         double* __restrict__ Cb, double* __restrict__ Rb,
+                                                         int* __restrict__ err) {
     __shared__ double a[GJ_B][GJ_B + 1];
     __shared__ double col[GJ_B];
     const uint32_t i = threadIdx.x / GJ_B, j = threadIdx.x % GJ_B;
-    a[i][j] = i < kb && j < kb ? D[(size_t)(k0 + i) * n + k0 + j] : i == j ? 1.0 : 0.0;
+    a[i][j] = i < kb && j < kb ? D[(size_t)(k0 + i) * n + k0 + j] : 0.0;
     __syncthreads();
     for (uint32_t k = 0; k < kb; k++) {
-        if (j == k) col[i] = a[i][k];  // column k before the update
+        if (j == k) {
+            col[i] = a[i][k];  // column k before the update
+            Cb[k * GJ_B + i] = a[i][k];
+        }
         __syncthreads();
         const double p = col[k];
         if (p == 0.0) {  // the same for every thread
@@ -1074,41 +1082,52 @@ __global__ void __launch_bounds__(GJ_B* GJ_B) k_gj_block(uint32_t n, uint32_t k0
             return;
         }
         const double piv = 1 / p, rkj = j == k ? piv : a[k][j] * piv, old = j == k ? 0.0 : a[i][j];
+        if (i == k) Rb[k * GJ_B + j] = rkj;
         __syncthreads();
         a[i][j] = i == k ? rkj : old - col[i] * rkj;
         __syncthreads();
     }
-    P[threadIdx.x] = a[i][j];
+    if (i < kb && j < kb) D[(size_t)(k0 + i) * n + k0 + j] = a[i][j];
 }
-// The block's rows (R and D), and the block's columns of the other rows (C).
-__global__ void __launch_bounds__(256) k_gj_panel(uint32_t n, uint32_t k0, uint32_t kb, double* __restrict__ D,
-                                                  const double* __restrict__ P, double* __restrict__ R,
-                                                  double* __restrict__ C) {
-    __shared__ double p[GJ_B * GJ_B];
-    for (uint32_t t = threadIdx.x; t < GJ_B * GJ_B; t += blockDim.x) p[t] = P[t];
+// The first half of the blocks: a thread takes a column through the block's rows;
+// the others: a thread takes a row through the block's columns.
+constexpr uint32_t GJ_P = 64;
+__global__ void __launch_bounds__(GJ_P) k_gj_panel(uint32_t n, uint32_t k0, uint32_t kb, double* __restrict__ D,
+                                                   const double* __restrict__ Cb, const double* __restrict__ Rb,
+                                                   double* __restrict__ R, double* __restrict__ C) {
+    __shared__ double m[GJ_B][GJ_B], piv[GJ_B];
+    const uint32_t nb = gridDim.x / 2;
+    const bool rows = blockIdx.x >= nb;
+    const double* src = rows ? Rb : Cb;
+    for (uint32_t t = threadIdx.x; t < GJ_B * GJ_B; t += GJ_P) m[t / GJ_B][t % GJ_B] = t / GJ_B < kb ? src[t] : 0.0;
+    if (threadIdx.x < GJ_B) piv[threadIdx.x] = threadIdx.x < kb ? Rb[threadIdx.x * GJ_B + threadIdx.x] : 0.0;
     __syncthreads();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const bool in = j >= k0 && j < k0 + kb;
+    const uint32_t q = (rows ? blockIdx.x - nb : blockIdx.x) * GJ_P + threadIdx.x;
+    if (q >= n) return;
+    const bool in = q >= k0 && q < k0 + kb;  // the block's own rows and columns are done
+    double* kept = rows ? C : R;
+    double* d = rows ? D + (size_t)q * n + k0 : D + (size_t)k0 * n + q;
+    const size_t step = rows ? 1 : n;
     double x[GJ_B];
 #pragma unroll
-    for (uint32_t t = 0; t < GJ_B; t++) x[t] = t < kb && !in ? D[(size_t)(k0 + t) * n + j] : 0.0;
-    for (uint32_t i = 0; i < GJ_B; i++) {
-        double s = 0;
-        if (in) {
-            s = p[i * GJ_B + (j - k0)];
-        } else {
+    for (uint32_t t = 0; t < GJ_B; t++) x[t] = !in && t < kb ? d[t * step] : 0.0;
 #pragma unroll
-            for (uint32_t t = 0; t < GJ_B; t++) s = __fma_rn(p[i * GJ_B + t], x[t], s);
-        }
-        R[(size_t)i * n + j] = i < kb ? s : 0.0;
+    for (uint32_t k = 0; k < GJ_B; k++) {
+        // of a column: the scaled row's entry; of a row: the pivot column's entry
+        const double f = rows ? x[k] : x[k] * piv[k];
+        kept[(size_t)k * n + q] = f;
+#pragma unroll
+        for (uint32_t t = 0; t < GJ_B; t++)
+            if (t != k) x[t] = x[t] - m[k][t] * f;
+        x[k] = rows ? 0.0 - f * piv[k] : f;
     }
-    // row j's entries in the block's columns (the block's own rows have none)
-    for (uint32_t t = 0; t < GJ_B; t++) C[(size_t)t * n + j] = !in && t < kb ? D[(size_t)j * n + k0 + t] : 0.0;
+#pragma unroll
+    for (uint32_t t = 0; t < GJ_B; t++)
+        if (!in && t < kb) d[t * step] = x[t];
 }
-// D = (D without the block's columns) - C R on the other rows, R on the block's.
-__global__ void __launch_bounds__(256) k_gj_update(uint32_t n, uint32_t k0, uint32_t kb, double* __restrict__ D,
-                                                   const double* __restrict__ R, const double* __restrict__ C) {
+// D -= C R, pivot by pivot (zero in the block's own rows and columns).
+__global__ void __launch_bounds__(256) k_gj_update(uint32_t n, double* __restrict__ D, const double* __restrict__ R,
+                                                   const double* __restrict__ C) {
     __shared__ double sr[GJ_B][GJ_T], sc[GJ_B][GJ_T];
     const uint32_t i0 = blockIdx.y * GJ_T, j0 = blockIdx.x * GJ_T;
     for (uint32_t t = threadIdx.x; t < GJ_B * GJ_T; t += 256) {
@@ -1116,9 +1135,16 @@ __global__ void __launch_bounds__(256) k_gj_update(uint32_t n, uint32_t k0, uint
         sr[k][c] = j0 + c < n ? R[(size_t)k * n + j0 + c] : 0.0;
         sc[k][c] = i0 + c < n ? C[(size_t)k * n + i0 + c] : 0.0;
     }
-    __syncthreads();
     const uint32_t tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double acc[4][4] = {};
+    double acc[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const uint32_t i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
+            acc[u][v] = i < n && j < n ? D[(size_t)i * n + j] : 0.0;
+        }
+    __syncthreads();
 #pragma unroll 8
     for (uint32_t k = 0; k < GJ_B; k++) {
         double a[4], b[4];
@@ -1130,17 +1156,14 @@ __global__ void __launch_bounds__(256) k_gj_update(uint32_t n, uint32_t k0, uint
 #pragma unroll
         for (int u = 0; u < 4; u++)
 #pragma unroll
-            for (int v = 0; v < 4; v++) acc[u][v] = __fma_rn(a[u], b[v], acc[u][v]);
+            for (int v = 0; v < 4; v++) acc[u][v] = acc[u][v] - a[u] * b[v];
     }
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
         for (int v = 0; v < 4; v++) {
             const uint32_t i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
-            if (i >= n || j >= n) continue;
-            double* d = D + (size_t)i * n + j;
-            if (i >= k0 && i < k0 + kb) *d = R[(size_t)(i - k0) * n + j];
-            else *d = (j >= k0 && j < k0 + kb ? 0.0 : *d) - acc[u][v];
+            if (i < n && j < n) D[(size_t)i * n + j] = acc[u][v];
         }
 }
 
@@ -2096,15 +2119,15 @@ static void build_direct(Level& li, cudaStream_t s) {
     if (!n) return;
     k_dense_from_csr<<<grid_for(n, 128), 128, 0, s>>>(n, li.A.ia.p, li.A.ja.p, li.A.a.p, li.cinv.p);
     CK_LAUNCH();
-    Tmp<double> P(GJ_B * GJ_B), R((size_t)GJ_B * n), C((size_t)GJ_B * n);
+    Tmp<double> Cb(GJ_B * GJ_B), Rb(GJ_B * GJ_B), R((size_t)GJ_B * n), C((size_t)GJ_B * n);
     Tmp<int> err(1);
     err.zero(s);
     const unsigned nt = (n + GJ_T - 1) / GJ_T;
     for (uint32_t k = 0; k < n; k += GJ_B) {
         const uint32_t kb = std::min(GJ_B, n - k);
-        k_gj_block<<<1, GJ_B * GJ_B, 0, s>>>(n, k, kb, li.cinv.p, P.p, err.p);
-        k_gj_panel<<<grid_for(n, 256), 256, 0, s>>>(n, k, kb, li.cinv.p, P.p, R.p, C.p);
-        k_gj_update<<<dim3(nt, nt), 256, 0, s>>>(n, k, kb, li.cinv.p, R.p, C.p);
+        k_gj_block<<<1, GJ_B * GJ_B, 0, s>>>(n, k, kb, li.cinv.p, Cb.p, Rb.p, err.p);
+        k_gj_panel<<<2 * grid_for(n, GJ_P), GJ_P, 0, s>>>(n, k, kb, li.cinv.p, Cb.p, Rb.p, R.p, C.p);
+        k_gj_update<<<dim3(nt, nt), 256, 0, s>>>(n, li.cinv.p, R.p, C.p);
     }
     CK_LAUNCH();
     if (read_flag(err.p, s)) MLP_THROW(ERR_INTERNAL, "zero pivot in the coarse-level inverse");
