@@ -60,14 +60,23 @@ MSPLIT = dict(q=(0.8,), niter=(5,), max_levels=15, degree_max=2, order="simple_1
 # uh_cheb as `ml_prec -p uh_cheb -s 3 -b 4` runs it: sigma 3, Chebyshev degree 4
 UH_CHEB = dict(sigma=(3.0,), ncheb=(4,), use_tails=True)
 # DRAM bytes of one level-0 SpMV launch on this matrix from an ncu capture
-# (102.99 MB read + 2.94 MB written): the slices and x stream once; most of y
+# (102.98 MB read + 3.91 MB written): the slices and x stream once; most of y
 # is still in L2 when the kernel ends.
-SPMV_DRAM_TRAFFIC = 105.93e6
+SPMV_DRAM_TRAFFIC = 106.89e6
+SPMV_COPIES = 8
 # DRAM bytes (read + write) of one launch of a composed sweep (k_state_step) on
 # this matrix, from the ncu captures summarised in
 # profiles/sweeps_60x220x85.md (cold caches: in the graph its operators stay
 # in L2). Not measured in the run.
 SWEEP_DRAM_TRAFFIC = {"sweep L2": 9.32e6, "sweep L1": 34.57e6}
+
+
+def spmv_bytes(ia):
+    """Bytes of y = A x in slices of 32 rows: 12 a slot (a slice is as wide as its
+    longest row), a word a slice, x and y."""
+    lens = np.diff(ia.astype(np.int64))
+    wide = np.pad(lens, (0, -len(lens) % 32)).reshape(-1, 32).max(axis=1)
+    return int(12 * 32 * wide.sum() + 4 * (len(wide) + 1) + 16 * len(lens))
 
 
 def dist_env():
@@ -381,8 +390,7 @@ def run_ours(args, ws, rank, local):
     del fa, za
     # the PCG's own launches inside the solve graph (mlp_pcg_timeline, one
     # iteration near the end), with their algorithmic bytes
-    nnz = A.nnz()
-    pcg_bytes = {"pcg spmv_dot": 12 * nnz + 4 * (N + 1) + 16 * N, "pcg update": 48 * N, "pcg dot_rz": 16 * N,
+    pcg_bytes = {"pcg spmv_dot": spmv_bytes(A.arrays()[0]), "pcg update": 48 * N, "pcg dot_rz": 16 * N,
                  "pcg p": 24 * N}
     out["pcg_timeline"] = [[nm, us_, pcg_bytes[nm]] for nm, us_ in Pp.pcg_timeline(A, b_d, x_d, EPS)
                            if nm in pcg_bytes]
@@ -440,34 +448,33 @@ def run_ours(args, ws, rank, local):
                               params="sigma 3, degree 4 per level, tails (-p uh_cheb -s 3 -b 4)")
         progress("uh_cheb steps")
 
-    # ---- roofline: level-0 SpMV (staged kernel), events on its stream ----
-    # 50 launches back to back between two events, alternating between two
-    # copies of the matrix and vectors (2 x 116 MB > the 126 MB L2), so every
+    # ---- roofline: level-0 SpMV (sliced rows), events on its stream ----
+    # 48 launches back to back between two events, in turn on SPMV_COPIES copies
+    # of the matrix and vectors (8 x 112 MB, seven times the 126 MB L2: with two
+    # copies part of each was still there when its turn came), so every
     # launch streams its matrix from HBM and the launch latency is amortised.
     ia, ja, a = A.arrays()
-    A2 = M.CSRMatrix.from_arrays(ia, ja, a)
-    mats = [A, A2]
-    xs = [torch.randn(N, dtype=torch.float64, device=dev) for _ in range(2)]
-    ys = [torch.empty_like(xs[0]) for _ in range(2)]
+    mats = [A] + [M.CSRMatrix.from_arrays(ia, ja, a) for _ in range(SPMV_COPIES - 1)]
+    xs = [torch.randn(N, dtype=torch.float64, device=dev) for _ in range(SPMV_COPIES)]
+    ys = [torch.empty_like(xs[0]) for _ in range(SPMV_COPIES)]
 
-    def spmv(k):
-        check(lib().mlp_spmv(mats[k & 1].h, C.c_void_p(xs[k & 1].data_ptr()), C.c_void_p(ys[k & 1].data_ptr()),
-                             C.c_void_p(stream.cuda_stream)))
+    def spmv(k, s):
+        k %= SPMV_COPIES
+        check(lib().mlp_spmv(mats[k].h, C.c_void_p(xs[k].data_ptr()), C.c_void_p(ys[k].data_ptr()), C.c_void_p(s)))
 
-    for k in range(6):
-        spmv(k)
+    for k in range(2 * SPMV_COPIES):
+        spmv(k, stream.cuda_stream)
     torch.cuda.synchronize()
     # the launches are recorded into a CUDA graph so that the host's call
     # overhead does not pace them
-    reps = 50
+    reps = 6 * SPMV_COPIES
     graph = torch.cuda.CUDAGraph()
     cap = torch.cuda.Stream(dev)
     with torch.cuda.stream(cap):
         cs = cap.cuda_stream
         graph.capture_begin()
         for k in range(reps):
-            check(lib().mlp_spmv(mats[k & 1].h, C.c_void_p(xs[k & 1].data_ptr()), C.c_void_p(ys[k & 1].data_ptr()),
-                                 C.c_void_p(cs)))
+            spmv(k, cs)
         graph.capture_end()
     graph.replay()
     torch.cuda.synchronize()
@@ -482,8 +489,8 @@ def run_ours(args, ws, rank, local):
     out["spmv_ms"] = e0.elapsed_time(e1) / reps
     progress("level-0 SpMV")
     del graph
-    out["spmv_bytes"] = 12 * A.nnz() + 4 * (N + 1) + 8 * N + 8 * N
-    del A2
+    out["spmv_bytes"] = spmv_bytes(ia)
+    del mats, xs, ys
 
     if not args.no_forms:
         # ---- e2e through the C ABI with host buffers ----
@@ -755,8 +762,8 @@ def main():
                      "spmv_level0": {"kernel": "level-0 SpMV y = A x (k_spmv_sell, rows in slices of 32)",
                                      "achieved": achieved, "frac": achieved / hbm,
                                      "bytes_per_launch": res["spmv_bytes"], "ms_per_launch": res["spmv_ms"],
-                                     "timing": "50 launches back to back in one CUDA graph, two matrix copies "
-                                               "alternated (232 MB > L2)",
+                                     "timing": f"{6 * SPMV_COPIES} launches back to back in one CUDA graph, "
+                                               f"{SPMV_COPIES} matrix copies in turn (seven times the L2)",
                                      "traffic": SPMV_DRAM_TRAFFIC,
                                      "traffic_source": "taken from profiles/spmv_level0_60x220x85.md (an ncu capture "
                                                        "of one launch on this matrix), not measured in this run"}},

@@ -229,7 +229,8 @@ __device__ __forceinline__ void spmv_pipe(uint32_t n, const uint32_t* __restrict
 // then its eight gathers are in flight together. The tile pipeline above reads
 // a row's values with a stride between the lanes, which holds it at the L1's
 // rate: in the PCG iteration at 60x220x85 the SpMV with (Ap, p) took 33 us there
-// against 23.6 here, and the SpMV alone 25.2 against 18.0 us (6.4 TB/s). The
+// against 23.6 here, and the SpMV alone, repeated on one matrix, 25.2 against 18.0 us
+// (19.2 over copies that have left L2: 5.84 TB/s). The
 // matrix is read once an iteration and is larger than what L2 can keep beside
 // the preconditioner, so its loads are marked streaming.
 // Unused entries have the column SELL_NONE.
@@ -3688,9 +3689,11 @@ static void record_direction(Prec& P, uint32_t n, bool flexible, cudaStream_t s)
 
 // Iterations per pass of the loop: a pass costs 7 us by itself (60x220x85), one
 // iteration of it more than needed is run every other solve and changes
-// nothing (skip). With short plans two are worth it (six launches: 38
-// iterations, 19 passes less, against half an application and its PCG kernels);
-// with 31 launches an application costs as much as the passes saved.
+// nothing (skip). Solves with one -> two iterations a pass, mean over stops at
+// 1e-7 to 1e-10 (odd and even counts): plans of 2 launches 0.82 -> 0.76 ms
+// (30x40x20 iid), 6 launches 1.45 -> 1.39 (60x220x20 iid), 11 launches 1.29 ->
+// 1.19 and 1.40 -> 1.35 (30x60x20, 40x80x20 layered), but 31 launches 3.28 -> 3.34
+// (60x220x20 layered), 51 launches 4.79 -> 4.84 and 151 launches 20.6 -> 20.8.
 static constexpr size_t LOOP_TWICE_MAX = 12;
 static uint32_t loop_iterations(const Prec& P) { return P.plan.launches <= LOOP_TWICE_MAX ? 2 : 1; }
 // Iterations that a solve of it runs: the first advance, then whole passes.

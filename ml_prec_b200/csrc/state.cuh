@@ -61,14 +61,26 @@ struct StateOps {
 // must hold their dropped-link values). C (cn x cn, row-major, FP64) is the
 // dense operator of level m + 1, or null. Up to ABSORB_WHOLE rows it becomes
 // part of K_m and G as any other factor; not in an FP32 hierarchy, whose coarse
-// solve keeps FP64 entries and sums (60x220x20 iid, 4 coarse rows: one launch
-// more, 24.5 us an application in place of 23). Larger, K_m's rows with coarse
-// columns (nd of them) take their product with it as a dense part, K_C C,
-// where that is at most ABSORB_DENSE bytes: a sweep then reads nd x cn entries
-// but needs no coarse launch (without a system, m = 0, G's rows do). At level 2 of the 60x220x85 field (cn = 422, nd =
-// 2,292, 7.7 MB that stay in L2) a sweep takes 3.0 us of the chain in place of
-// 4.6 for the sweep and its coarse launch. Past it (c = 0.1: cn = 1,317, 84 MB)
-// the sweeps call the coarse operator. Returns null when a row of an operator
+// solve keeps FP64 entries and sums (one launch more a call of system m:
+// 60x220x20 iid, 4 coarse rows, 24.5 us an application in place of 23). Larger,
+// K_m's rows with coarse columns (nd of them) take their product with it as a
+// dense part, K_C C, where that is at most ABSORB_DENSE bytes and ABSORB_DENSE_N
+// columns: a sweep then reads nd x cn entries but needs no coarse launch (without
+// a system, m = 0, G's rows do). Past it the sweeps call the coarse operator.
+// An application's launches in a graph, FP64, us (fields layered, or iid where
+// said so; other levels tabulated than by default in the lines marked *):
+//   cn                              whole   dense part   separate
+//    4  60x220x20 iid                12.5      14.4
+//   18  60x220x85 iid                18.5      18.5
+//   31  59x211x37, c = 0.1 *         1250      1430
+//   58  30x40x20, c = 0.1 *           230       285          422
+//   76  60x110x40, c = 0.3 *          259       319          445
+//  138  60x220x85, c = 0.3            521       503          657
+//  204  60x220x20                     100        78          101
+//  422  60x220x85 (nd = 2,292)        262       129          154
+// so a whole absorption pays up to somewhere near 100 rows (32 keeps well inside
+// it: its fill grows with nd), a dense part wherever it fits the registers.
+// Returns null when a row of an operator
 // holds more than STATE_ROW_MAX entries. fp32: the sparse values are stored in
 // FP32, rounded once from their FP64 products.
 constexpr uint32_t STATE_ROW_MAX = 1024;
