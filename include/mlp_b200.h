@@ -122,7 +122,8 @@ int mlp_set_device(int device);
 
 /* ---- matrices ------------------------------------------------------------
  * Replaces CSRMatrix / SkylineMatrix storage (matrix.h:187-291): uint32 ia
- * (n+1), ja and FP64 a (nnz), diagonal first in every row. The library keeps a
+ * (n+1), ja and FP64 a (nnz), diagonal first in every row; a row may hold a
+ * column more than once, its entries then add up. The library keeps a
  * device copy; the host arrays may be released after the call. */
 int mlp_matrix_create(uint32_t n, const uint32_t* ia_host, const uint32_t* ja_host, const double* a_host,
                       mlp_matrix** out);
